@@ -42,7 +42,8 @@ class State(NamedTuple):
 
 def _dev(x, dtype) -> torch.Tensor:
     if isinstance(x, torch.Tensor):
-        return x.to(device="cuda", dtype=dtype).contiguous()
+        # the engine reads the storage: a lazily conjugated or negated view is written out
+        return x.to(device="cuda", dtype=dtype).contiguous().resolve_conj().resolve_neg()
     return torch.from_numpy(np.ascontiguousarray(np.asarray(x))).to(device="cuda", dtype=dtype)
 
 

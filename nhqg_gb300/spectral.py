@@ -66,7 +66,7 @@ def _planes(x) -> torch.Tensor:
         t = torch.from_numpy(np.ascontiguousarray(np.asarray(x, dtype=np.complex128))).to("cuda")
     if t.dim() == 2:
         t = t.unsqueeze(0)
-    return t.contiguous()
+    return t.contiguous().resolve_conj().resolve_neg()
 
 
 def _host(a):
