@@ -19,7 +19,7 @@ import torch
 from . import _native as nat
 from .engine import Engine, _stream_handle, require_cuda
 from .grid import Grid
-from .solver import State, to_device
+from .solver import State, _check_status, to_device
 
 
 class Ensemble:
@@ -75,14 +75,20 @@ class Ensemble:
         d = self.engines[i].state_desc(*s)
         nat.check(self.lib.nhqg_batch_load(self.handle, int(i), ctypes.byref(d), _stream_handle()),
                   "nhqg_batch_load")
-        st = self.engines[i].device_status(reset=True)
-        if st & nat.DEVICE_STATUS_OOB:
+        if _check_status(self.engines[i], f"Ensemble.load({i})") & nat.DEVICE_STATUS_OOB:
             raise ValueError("Ensemble.load: the state has content outside the 2/3 band")
 
     def step(self, n_steps: int = 1) -> None:
         """Advance every member by n_steps (stream-ordered, no host sync)."""
         nat.check(self.lib.nhqg_batch_step(self.handle, int(n_steps), _stream_handle()),
                   "nhqg_batch_step")
+
+    def check(self) -> None:
+        """Synchronise and raise if a wait inside a kernel ran out of time in any
+        member's steps since the last check or load."""
+        torch.cuda.synchronize()
+        for i, e in enumerate(self.engines):
+            _check_status(e, f"Ensemble member {i}")
 
     def store(self, i: int) -> State:
         g = self.grids[i]

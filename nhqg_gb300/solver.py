@@ -67,9 +67,20 @@ def _copy(state) -> State:
     return State(*(t.clone() for t in s))
 
 
-def _check_band(eng, what: str) -> None:
+def _check_status(eng, what: str) -> int:
+    """Read and clear the device status; raises on a kernel wait that ran out
+    (its results are incomplete, since whichever call left it)."""
     st = eng.device_status(reset=True)
-    if st & nat.DEVICE_STATUS_OOB:
+    if st < 0:
+        raise nat.NativeError(f"{what}: the device status could not be read")
+    if st & nat.DEVICE_STATUS_TIMEOUT:
+        raise RuntimeError(f"{what}: a wait inside a kernel ran out of time; the results of this and of "
+                           "earlier unchecked calls on this grid are incomplete")
+    return st
+
+
+def _check_band(eng, what: str) -> None:
+    if _check_status(eng, what) & nat.DEVICE_STATUS_OOB:
         raise ValueError(
             f"{what}: the state has content outside the 2/3 band; the GPU step "
             "assumes band-limited input (apply sanitize_state first)")
@@ -81,7 +92,7 @@ def sanitize_state(state, grid: Grid) -> State:
     eng = engine_for(grid)
     s = _copy(state)
     eng.sanitize(*s)
-    eng.device_status(reset=True)
+    _check_status(eng, "sanitize_state")
     return s
 
 
@@ -89,7 +100,8 @@ def step_inplace(state: State, grid: Grid, n_steps: int = 1, check: bool = False
                  precision: str = "fp64") -> State:
     """Advance ``state`` (CUDA tensors, reference layout) by ``n_steps``
     imex_step applications in place; stream-ordered, no host sync unless
-    ``check`` (then the band-limit status is verified)."""
+    ``check`` (then the status of this and of earlier unchecked calls is
+    verified: the band limit, and waits inside kernels)."""
     eng = engine_for(grid)
     eng.step(*state, n_steps=n_steps, precision=precision)
     if check:
@@ -255,6 +267,7 @@ def run(grid: Grid, state, n_steps: int, save_interval: int, use_imex: bool = Tr
     rem = n_steps % save_interval
     if rem:
         step_inplace(s, grid, rem, check=(n_outer == 0), precision=precision)
+    _check_status(engine_for(grid), "run")  # the chunks after the first
     return s, snaps
 
 
