@@ -175,6 +175,7 @@ int nhqg_ctx_create(const nhqg_grid_desc* g, nhqg_ctx** out) {
   p.d = make_dims(g->Nx, g->Nz, pad32);
   p.plan = plan;
   p.plan_v = make_fft_plan(g->Nz);
+  p.plan_vh = make_fft_plan(g->Nz / 2);
   p.fast_dct = g->Nz % 2 == 0 && p.plan_v.npass > 0 && getenv("NHQG_DENSE_VERTICAL") == nullptr;
   p.advection = g->advection;
   p.closure = g->thermal_closure;
@@ -342,11 +343,15 @@ int nhqg_ctx_create(const nhqg_grid_desc* g, nhqg_ctx** out) {
   {
     const char* off = getenv("NHQG_FX_VERTICAL");
     if (p.fast_dct && N <= 512 && !(off && off[0] == '0')) {
-      std::vector<fx::cfx> tw = fx_roots(N, N), cs = fx_roots(N + 1, 2 * N);
+      const int n = N / 2;
+      std::vector<fx::cfx> tw = fx_roots(n, n), cs = fx_roots(N + 1, 2 * N);
+      std::vector<int> perm(n);
+      make_fft_perm(p.plan_vh, perm.data());
       for (fx::cfx& v : tw) v.y = -v.y;
       for (fx::cfx& v : cs) v.y = -v.y;
       UP(t.fx.tw_v, tw.data(), tw.size());
       UP(t.fx.cs_v, cs.data(), cs.size());
+      UP(t.fx.perm_v, perm.data(), perm.size());
     }
   }
 

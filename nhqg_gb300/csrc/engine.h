@@ -131,8 +131,10 @@ struct Tables {
     long long *sponge = nullptr, *eta = nullptr;
     int sponge_e = 0;
     int* eta_e = nullptr;
-    // vertical DCT (null: FP64): exp(-2 pi i k / Nz) [Nz], exp(-i pi j / Nz) [Nz+1]
+    // vertical DCT (null: FP64) by FFTs of length n = Nz/2: exp(-2 pi i k / n) [n],
+    // exp(-i pi j / Nz) [Nz+1], positions of the frequencies [n]
     fx::cfx *tw_v = nullptr, *cs_v = nullptr;
+    int* perm_v = nullptr;
   } fx;
 };
 
@@ -140,6 +142,7 @@ struct Params {
   Dims d;
   FftPlan plan;
   FftPlan plan_v;  // length Nz (DCT-I); npass <= 0 -> dense vertical transforms
+  FftPlan plan_vh;  // length Nz/2 (the fixed-point DCT-I)
   FftPlan plan_nx; // length Nx (physical-space diagnostics)
   bool fast_dct;
   int advection, closure, exchange, wbc, substeps;
@@ -184,8 +187,11 @@ inline col::Dct make_dct(const Params& p, const Tables& t) {
   d.perm = t.perm_v;
   d.V = t.V;
   d.Vinv = t.Vinv;
+  d.plan_h = p.plan_vh;
+  d.m_h = Div::magic(p.d.Nz / 2);
   d.tw_fx = t.fx.tw_v;
   d.cs_fx = t.fx.cs_v;
+  d.perm_h = t.fx.perm_v;
   return d;
 }
 
