@@ -598,7 +598,8 @@ int nhqg_ctx_create(const nhqg_grid_desc* g, nhqg_ctx** out) {
     if (shell_tc_supported(G)) {
       // packed on the device, a few matrices at a time through a staging buffer
       if (dalloc(c, &t.shell_fx, t.n_shells * shell_tc_elems(G)) != cudaSuccess ||
-          dalloc(c, &t.shell_rowe, t.n_shells * shell_tc_rows(G)) != cudaSuccess)
+          dalloc(c, &t.shell_rowe, t.n_shells * shell_tc_rows(G)) != cudaSuccess ||
+          dalloc(c, &t.shell_diag, t.n_shells * shell_tc_rows(G)) != cudaSuccess)
         return fail(NHQG_ERR_CUDA);
       const int batch = (int)std::max<size_t>(1, std::min<size_t>(t.n_shells, ((size_t)8 << 20) / gg));
       double* stage = nullptr;
@@ -614,7 +615,8 @@ int nhqg_ctx_create(const nhqg_grid_desc* g, nhqg_ctx** out) {
         }
         if (err == cudaSuccess)
           err = launch_shell_pack(stage, t.shell_fx + (size_t)s0 * shell_tc_elems(G),
-                                  t.shell_rowe + (size_t)s0 * shell_tc_rows(G), n, G, nullptr);
+                                  t.shell_rowe + (size_t)s0 * shell_tc_rows(G),
+                                  t.shell_diag + (size_t)s0 * shell_tc_rows(G), n, G, nullptr);
         if (err == cudaSuccess) err = cudaDeviceSynchronize();  // the staging buffer is rewritten
       }
       cudaFree(stage);

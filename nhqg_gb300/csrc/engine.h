@@ -111,9 +111,11 @@ struct Tables {
   double* cc = nullptr;
   // shells
   double* shell_inv = nullptr;  // [n_shells*G*G], only where shell_tc_supported(G) is false
-  // biased integers [n_shells][Kp/2][Gr][2] and row exponents [n_shells][Gr] (csrc/shell_tc.cu)
+  // biased integers [n_shells][Kp/2][Gr][2], row exponents and diagonals [n_shells][Gr]
+  // (csrc/shell_tc.cu)
   unsigned long long* shell_fx = nullptr;
   int* shell_rowe = nullptr;
+  double* shell_diag = nullptr;
   int* shell_start = nullptr;   // [n_shells+1]
   int* shell_modes = nullptr;   // [M]
   int n_shells = 0;
@@ -391,7 +393,7 @@ cudaError_t launch_shell(const Params& p, const Tables& t, const Work& w, const 
 bool shell_tc_supported(int G);
 size_t shell_tc_elems(int G);  // integers of one packed matrix
 size_t shell_tc_rows(int G);   // row exponents of one matrix
-cudaError_t launch_shell_pack(const double* src, unsigned long long* tab, int* rowe, int n, int G,
+cudaError_t launch_shell_pack(const double* src, unsigned long long* tab, int* rowe, double* diag, int n, int G,
                               cudaStream_t st);
 cudaError_t launch_shell_tc(const Params& p, const Tables& t, const Work& w, const double2* rhs_w,
                             double2* w_out, cudaStream_t st);
