@@ -53,15 +53,21 @@ std::vector<int> horizontal_fx_twiddles(int N) {
   return out;
 }
 
-// v * s as integers, each run of `run` values at one exponent above every |v s|
+// v * s as integers, each run of `run` values at one exponent above every |v s|;
+// a run with an infinity or a NaN gets kENan
 void horizontal_fx_table(const std::vector<double>& v, double s, size_t run, std::vector<long long>& out,
                          std::vector<int>& e) {
   out.resize(v.size());
   e.assign(v.size() / run, -900);
   for (size_t b = 0; b < e.size(); ++b) {
     double m = 0.0;
-    for (size_t i = b * run; i < (b + 1) * run; ++i) m = std::max(m, std::fabs(v[i] * s));
-    if (m > 0.0) std::frexp(m, &e[b]);
+    bool finite = true;
+    for (size_t i = b * run; i < (b + 1) * run; ++i) {
+      finite = finite && std::isfinite(v[i] * s);
+      m = std::max(m, std::fabs(v[i] * s));
+    }
+    if (!finite) e[b] = fx::kENan;
+    else if (m > 0.0) std::frexp(m, &e[b]);
     e[b] += 1;
     for (size_t i = b * run; i < (b + 1) * run; ++i) out[i] = fx::to_fx(v[i] * s, e[b]);
   }
