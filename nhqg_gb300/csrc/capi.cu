@@ -936,8 +936,8 @@ int to_nodal_f32(nhqg_ctx* c, const double2* q, const double2* w, const double2*
   return NHQG_OK;
 }
 
-int horizontal_step(nhqg_ctx* c, const double2* qn, const double2* wn, const double2* tn,
-                    cudaStream_t st) {
+// the step's FP64 products
+HorizArgs step_products(const nhqg_ctx* c, const double2* qn, const double2* wn, const double2* tn) {
   const Params& p = c->p;
   HorizArgs a{};
   a.form = p.advection == NHQG_ADV_JACOBIAN ? HF_JAC : HF_FLUX;
@@ -949,7 +949,12 @@ int horizontal_step(nhqg_ctx* c, const double2* qn, const double2* wn, const dou
   a.levels = p.d.P;
   a.psi = nullptr; a.q = qn; a.w = wn; a.th = tn;
   a.Aq = c->Aq; a.Aw = c->Aw; a.Ath = c->At;
-  CK(launch_horizontal(p, c->t, c->w, a, st, &c->launches));
+  return a;
+}
+
+int horizontal_step(nhqg_ctx* c, const double2* qn, const double2* wn, const double2* tn,
+                    cudaStream_t st) {
+  CK(launch_horizontal(c->p, c->t, c->w, step_products(c, qn, wn, tn), st, &c->launches));
   return NHQG_OK;
 }
 
@@ -1672,7 +1677,8 @@ int nhqg_autotune(nhqg_ctx* c, void* stream) {
   for (int pi = 0; pi < 2; ++pi) {
     const bool f32 = pi == 1;
     if (f32 && !c->Qf) continue;  // FP32 buffers exist once the mixed path is enabled
-    if (!f32 && c->t.fx.tw) continue;  // the fixed-point products have no tiles to choose
+    // the fixed-point products have no tiles to choose
+    if (!f32 && horizontal_fx_takes(c->p, c->t, c->w, step_products(c, c->Qn, c->Wn, c->Tn))) continue;
     const int* cols = f32 ? col32 : col64;
     const int* rows = f32 ? row32 : row64;
     const int nc = f32 ? 5 : 4, nr = 4;
