@@ -268,6 +268,23 @@ int nhqg_triple_advection_32(nhqg_ctx *ctx, int advection, int levels,
 int nhqg_sponge_product_32(nhqg_ctx *ctx, int levels, const void *f, void *out,
                            void *stream);
 
+/* The plane products (the context's rule) with a workspace that the caller
+ * lends for the call: device memory, 16-byte aligned, free for reuse once the
+ * call's work on the stream is done.  The calls above run in chunks of the few
+ * levels that the context's step buffers hold; with
+ * nhqg_plane_workspace_bytes(ctx, NHQG_ADV_* or NHQG_PLANE_SPONGE, levels, &n) bytes
+ * they take all levels at once (up to 256 MiB of intermediates per chunk).  0
+ * means that the context's own buffers hold as much; a null or smaller workspace
+ * is not used.  Nothing is allocated or kept. */
+enum { NHQG_PLANE_SPONGE = 2 };
+int nhqg_plane_workspace_bytes(const nhqg_ctx *ctx, int advection, int levels, size_t *bytes);
+int nhqg_triple_advection_ws(nhqg_ctx *ctx, int advection, int levels,
+                             const void *psi, const void *q, const void *w,
+                             const void *th, void *Aq, void *Aw, void *Ath,
+                             void *workspace, size_t workspace_bytes, void *stream);
+int nhqg_sponge_product_ws(nhqg_ctx *ctx, int levels, const void *f, void *out,
+                           void *workspace, size_t workspace_bytes, void *stream);
+
 /* sanitize_state (nhqg/solver.py:128-146), in place: Hermitian projection
  * of the ky=0 column and the 2/3 band limit (2/3 rule), or of the ky=0 and
  * ky=Nx/2 columns (3/2 rule, no band limit). */

@@ -37,6 +37,7 @@ DEVICE_STATUS_OOB = 1 << 0
 DEVICE_STATUS_TIMEOUT = 1 << 1
 
 ADV = {"flux": 0, "jacobian": 1}
+PLANE_SPONGE = 2
 CLOSURE = {"fixed_conduction": 0, "evolve_mean": 1}
 EXCHANGE = {"legacy": 0, "balanced_sbp2": 1, "balanced_sbp2_pc": 2}
 WBC = {"dirichlet": 0, "neumann": 1}
@@ -155,6 +156,12 @@ SIGNATURES = {
                                  [ctypes.c_void_p] * 7 + [ctypes.c_void_p]),
     "nhqg_sponge_product_32": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p,
                                               ctypes.c_void_p, ctypes.c_void_p]),
+    "nhqg_plane_workspace_bytes": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int,
+                                                  ctypes.POINTER(ctypes.c_size_t)]),
+    "nhqg_triple_advection_ws": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int] +
+                                 [ctypes.c_void_p] * 8 + [ctypes.c_size_t, ctypes.c_void_p]),
+    "nhqg_sponge_product_ws": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int] + [ctypes.c_void_p] * 3 +
+                               [ctypes.c_size_t, ctypes.c_void_p]),
     "nhqg_sanitize": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(StateDesc), ctypes.c_void_p]),
     "nhqg_mean_temp_solve": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                             ctypes.c_int, ctypes.c_void_p]),

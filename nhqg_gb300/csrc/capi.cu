@@ -42,12 +42,6 @@ struct nhqg_ctx {
   // learned closure (null weights: off) and its tendency buffer [P*M]
   ClosureModel closure{};
   double2* Cq = nullptr;
-  // workspace of the plane API (PlaneWork); x1 null until its first use
-  struct PlaneBufs {
-    double2 *x1 = nullptr, *x2 = nullptr;
-    size_t x1_elems = 0, x2_elems = 0;
-    int *e1 = nullptr, *e2 = nullptr;
-  } plane;
   // bumped whenever the launch sequence of a step changes (precision, tiles):
   // captured step graphs of a batch compare it
   unsigned version = 0;
@@ -725,10 +719,12 @@ int nhqg_ctx_create(const nhqg_grid_desc* g, nhqg_ctx** out) {
     const int ng = (p.advection == NHQG_ADV_JACOBIAN) ? 3 : (t.fx.sponge ? 9 : 6);
     w.x1_elems = (size_t)nf1 * P * d.Mc * d.Nh;
     w.x2_elems = (size_t)ng * P * d.Mc * d.Nh;
-    // the plane API (full Nk columns, up to 11 fields) reuses these in level chunks
-    const size_t plane_min = (size_t)11 * d.Nk * d.Nh;
+    // the plane API (full Nk columns, up to 11 fields) reuses these in level chunks; at
+    // least 8 MB each, so that the calls that host work bounds (17 levels at 48^2, 55 us)
+    // need no lent workspace (PlaneWork), which costs 10 us of it
+    const size_t plane_min = std::max((size_t)11 * d.Nk * d.Nh, ((size_t)8 << 20) / sizeof(double2));
     if (w.x1_elems < plane_min) w.x1_elems = plane_min;
-    const size_t plane2_min = (size_t)6 * d.Mc * d.Nh;
+    const size_t plane2_min = std::max((size_t)6 * d.Mc * d.Nh, ((size_t)8 << 20) / sizeof(double2));
     if (w.x2_elems < plane2_min) w.x2_elems = plane2_min;
     if (dalloc(c, &w.x1, w.x1_elems) != cudaSuccess) return fail(NHQG_ERR_CUDA);
     if (dalloc(c, &w.x2, w.x2_elems) != cudaSuccess) return fail(NHQG_ERR_CUDA);
@@ -1402,67 +1398,65 @@ int nhqg_mean_temp_solve(nhqg_ctx* c, const double* R, double* out, int closure,
 
 namespace {
 
-// Workspace of a plane call of `levels` levels, nf1 input and ng intermediate
-// fields per level.  A context made for planes holds a step's buffers for a few
-// levels only, and a chunk of 3 levels at 256^2 leaves half of the SMs without
-// a CTA (65 levels: 22 x 3 launches, 4.9 ms against 2.2 ms for all levels at
-// once).  So a context whose step buffers do not hold the call gets one larger
-// workspace, once, kept until it is destroyed: up to 256 MB of H1 output, 512
-// levels at most.  Under stream capture nothing is allocated, and where the
-// memory is short the step's buffers serve, in more chunks.
-struct PlaneWork {
-  nhqg_ctx* c;
-  bool swapped = false;
-  PlaneWork(nhqg_ctx* ctx, int levels, int nf1, int ng, cudaStream_t st) : c(ctx) {
+// Workspace of a plane call.  A context made for planes holds a step's buffers for
+// a few levels only, and a chunk of 3 levels at 256^2 leaves half of the SMs without
+// a CTA (65 levels: 22 x 3 launches, 4.9 ms against 2.2 ms for all levels at once).
+// So the caller may lend one for the length of the call, which the engine neither
+// keeps nor allocates: for the call's levels, up to 256 MB of H1 output and 512
+// levels; beyond that, and without one, the call runs in chunks of levels.
+struct PlaneShape {
+  int lev, nf1, ng;  // levels at once, input and intermediate fields per level
+  size_t x1, x2;     // elements
+  size_t n1, n2;     // exponents, one per H1 column and per H2 row pair
+
+  static constexpr size_t up(size_t bytes) { return (bytes + 255) / 256 * 256; }
+  PlaneShape(const nhqg_ctx* c, int advection, int levels) {
     const Dims& d = c->p.d;
-    const Work& w = c->w;
-    const size_t col1 = (size_t)d.Nk * d.Nh, col2 = (size_t)d.Mc * d.Nh;  // elements per level and field
-    if (w.x1_elems >= (size_t)levels * nf1 * col1 && w.x2_elems >= (size_t)levels * ng * col2) return;
-    if (!c->plane.x1 && !grow(col1, col2, st)) return;
-    exchange();
-    swapped = true;
+    nf1 = advection == NHQG_PLANE_SPONGE ? 1 : (advection == NHQG_ADV_JACOBIAN ? 8 : 5);
+    ng = advection == NHQG_PLANE_SPONGE ? 1 : (advection == NHQG_ADV_JACOBIAN ? 3 : 6);
+    const size_t col1 = (size_t)nf1 * d.Nk * d.Nh, col2 = (size_t)ng * d.Mc * d.Nh;
+    const size_t cap = std::max<size_t>(1, std::min<size_t>(512, ((size_t)256 << 20) / (col1 * sizeof(double2))));
+    lev = (int)std::min<size_t>(levels, cap);
+    x1 = lev * col1;
+    x2 = lev * col2;
+    n1 = c->w.e1 ? x1 / d.Nh : 0;
+    n2 = c->w.e2 ? x2 / (2 * (size_t)d.Mc) : 0;
+  }
+  // 0 where the context's own buffers hold as much
+  size_t bytes(const nhqg_ctx* c) const {
+    if (c->w.x1_elems >= x1 && c->w.x2_elems >= x2) return 0;
+    return up(x1 * sizeof(double2)) + up(x2 * sizeof(double2)) + up(n1 * sizeof(int)) + up(n2 * sizeof(int));
+  }
+};
+
+// the context's H1 / H2 buffers exchanged for the lent ones while it lives
+struct PlaneWork {
+  Work& w;
+  double2 *x1, *x2;
+  size_t x1_elems, x2_elems;
+  int *e1, *e2;
+  PlaneWork(nhqg_ctx* c, const PlaneShape& s, void* ws, size_t bytes)
+      : w(c->w), x1(w.x1), x2(w.x2), x1_elems(w.x1_elems), x2_elems(w.x2_elems), e1(w.e1), e2(w.e2) {
+    const size_t need = s.bytes(c);
+    if (!ws || need == 0 || bytes < need) return;
+    char* p = static_cast<char*>(ws);
+    auto take = [&](size_t n) { char* q = p; p += PlaneShape::up(n); return q; };
+    w.x1 = reinterpret_cast<double2*>(take(s.x1 * sizeof(double2)));
+    w.x2 = reinterpret_cast<double2*>(take(s.x2 * sizeof(double2)));
+    w.x1_elems = s.x1;
+    w.x2_elems = s.x2;
+    if (w.e1) {
+      w.e1 = reinterpret_cast<int*>(take(s.n1 * sizeof(int)));
+      w.e2 = reinterpret_cast<int*>(take(s.n2 * sizeof(int)));
+    }
   }
   ~PlaneWork() {
-    if (swapped) exchange();
+    w.x1 = x1; w.x2 = x2;
+    w.x1_elems = x1_elems; w.x2_elems = x2_elems;
+    w.e1 = e1; w.e2 = e2;
   }
   PlaneWork(const PlaneWork&) = delete;
   PlaneWork& operator=(const PlaneWork&) = delete;
-
- private:
-  bool grow(size_t col1, size_t col2, cudaStream_t st) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
-    // levels of the flux form (5 and 6 fields); the Jacobian (8 and 3) gets fewer
-    const size_t lev = std::min<size_t>(512, ((size_t)256 << 20) / (5 * col1 * sizeof(double2)));
-    if (lev * 5 * col1 <= c->w.x1_elems) return false;
-    nhqg_ctx::PlaneBufs n;
-    n.x1_elems = lev * 5 * col1;
-    n.x2_elems = lev * 6 * col2;
-    const size_t keep = c->allocs.size();
-    bool ok = dalloc(c, &n.x1, n.x1_elems) == cudaSuccess && dalloc(c, &n.x2, n.x2_elems) == cudaSuccess;
-    if (ok && c->w.e1)
-      ok = dalloc(c, &n.e1, n.x1_elems / c->p.d.Nh) == cudaSuccess &&
-           dalloc(c, &n.e2, n.x2_elems / (2 * (size_t)c->p.d.Mc)) == cudaSuccess;
-    if (!ok) {
-      cudaGetLastError();
-      while (c->allocs.size() > keep) {
-        cudaFree(c->allocs.back());
-        c->allocs.pop_back();
-      }
-      return false;
-    }
-    c->plane = n;
-    return true;
-  }
-  void exchange() {
-    Work& w = c->w;
-    std::swap(w.x1, c->plane.x1);
-    std::swap(w.x2, c->plane.x2);
-    std::swap(w.x1_elems, c->plane.x1_elems);
-    std::swap(w.x2_elems, c->plane.x2_elems);
-    std::swap(w.e1, c->plane.e1);
-    std::swap(w.e2, c->plane.e2);
-  }
 };
 
 // Plane APIs: products of caller-supplied nodal planes in the full rfft2
@@ -1470,19 +1464,19 @@ struct PlaneWork {
 // dealiasing rule (pad32) selects the 2/3 or the 3/2 products.
 int plane_advection(nhqg_ctx* c, bool pad32, int advection, int levels, const void* psi,
                     const void* q, const void* w, const void* th, void* Aq, void* Aw, void* Ath,
-                    void* stream) {
+                    void* ws, size_t ws_bytes, void* stream) {
   if (!c || levels <= 0 || !psi || !q || !w || !th || !Aq || !Aw || !Ath) return NHQG_ERR_BAD_ARG;
   if (advection != NHQG_ADV_FLUX && advection != NHQG_ADV_JACOBIAN) return NHQG_ERR_UNSUPPORTED;
   if (c->p.d.pad != pad32) return NHQG_ERR_UNSUPPORTED;
+  if ((uintptr_t)ws % sizeof(double2)) return NHQG_ERR_BAD_ARG;
   cudaStream_t st = S(stream);
   c->launches = 0;
   const Dims& d = c->p.d;
   const size_t plane = (size_t)d.Nx * d.Nk;
-  const int nf1 = advection == NHQG_ADV_JACOBIAN ? 8 : 5;
-  const int ng = advection == NHQG_ADV_JACOBIAN ? 3 : 6;
-  const PlaneWork pw(c, levels, nf1, ng, st);
-  int chunk = (int)std::min(c->w.x1_elems / ((size_t)nf1 * d.Nk * d.Nh),
-                            c->w.x2_elems / ((size_t)ng * d.Mc * d.Nh));
+  const PlaneShape sh(c, advection, levels);
+  const PlaneWork pw(c, sh, ws, ws_bytes);
+  int chunk = (int)std::min(c->w.x1_elems / ((size_t)sh.nf1 * d.Nk * d.Nh),
+                            c->w.x2_elems / ((size_t)sh.ng * d.Mc * d.Nh));
   if (chunk < 1) return NHQG_ERR_UNSUPPORTED;
   CK(cudaMemsetAsync(Aq, 0, (size_t)levels * plane * sizeof(double2), st));
   CK(cudaMemsetAsync(Aw, 0, (size_t)levels * plane * sizeof(double2), st));
@@ -1502,14 +1496,17 @@ int plane_advection(nhqg_ctx* c, bool pad32, int advection, int levels, const vo
   return NHQG_OK;
 }
 
-int plane_sponge(nhqg_ctx* c, bool pad32, int levels, const void* f, void* out, void* stream) {
+int plane_sponge(nhqg_ctx* c, bool pad32, int levels, const void* f, void* out, void* ws, size_t ws_bytes,
+                 void* stream) {
   if (!c || levels <= 0 || !f || !out) return NHQG_ERR_BAD_ARG;
   if (!c->p.has_sponge || c->p.d.pad != pad32) return NHQG_ERR_UNSUPPORTED;
+  if ((uintptr_t)ws % sizeof(double2)) return NHQG_ERR_BAD_ARG;
   cudaStream_t st = S(stream);
   c->launches = 0;
   const Dims& d = c->p.d;
   const size_t plane = (size_t)d.Nx * d.Nk;
-  const PlaneWork pw(c, levels, 1, 1, st);
+  const PlaneShape sh(c, NHQG_PLANE_SPONGE, levels);
+  const PlaneWork pw(c, sh, ws, ws_bytes);
   int chunk = (int)std::min(c->w.x1_elems / ((size_t)d.Nk * d.Nh), c->w.x2_elems / ((size_t)d.Mc * d.Nh));
   if (chunk < 1) return NHQG_ERR_UNSUPPORTED;
   CK(cudaMemsetAsync(out, 0, (size_t)levels * plane * sizeof(double2), st));
@@ -1534,21 +1531,42 @@ extern "C" {
 int nhqg_triple_advection_23(nhqg_ctx* c, int advection, int levels, const void* psi,
                              const void* q, const void* w, const void* th, void* Aq, void* Aw,
                              void* Ath, void* stream) {
-  return plane_advection(c, false, advection, levels, psi, q, w, th, Aq, Aw, Ath, stream);
+  return plane_advection(c, false, advection, levels, psi, q, w, th, Aq, Aw, Ath, nullptr, 0, stream);
 }
 
 int nhqg_triple_advection_32(nhqg_ctx* c, int advection, int levels, const void* psi,
                              const void* q, const void* w, const void* th, void* Aq, void* Aw,
                              void* Ath, void* stream) {
-  return plane_advection(c, true, advection, levels, psi, q, w, th, Aq, Aw, Ath, stream);
+  return plane_advection(c, true, advection, levels, psi, q, w, th, Aq, Aw, Ath, nullptr, 0, stream);
 }
 
 int nhqg_sponge_product_23(nhqg_ctx* c, int levels, const void* f, void* out, void* stream) {
-  return plane_sponge(c, false, levels, f, out, stream);
+  return plane_sponge(c, false, levels, f, out, nullptr, 0, stream);
 }
 
 int nhqg_sponge_product_32(nhqg_ctx* c, int levels, const void* f, void* out, void* stream) {
-  return plane_sponge(c, true, levels, f, out, stream);
+  return plane_sponge(c, true, levels, f, out, nullptr, 0, stream);
+}
+
+int nhqg_plane_workspace_bytes(const nhqg_ctx* c, int advection, int levels, size_t* bytes) {
+  if (!c || !bytes || levels <= 0 ||
+      (advection != NHQG_ADV_FLUX && advection != NHQG_ADV_JACOBIAN && advection != NHQG_PLANE_SPONGE))
+    return NHQG_ERR_BAD_ARG;
+  *bytes = PlaneShape(c, advection, levels).bytes(c);
+  return NHQG_OK;
+}
+
+int nhqg_triple_advection_ws(nhqg_ctx* c, int advection, int levels, const void* psi, const void* q,
+                             const void* w, const void* th, void* Aq, void* Aw, void* Ath, void* ws,
+                             size_t ws_bytes, void* stream) {
+  if (!c) return NHQG_ERR_BAD_ARG;
+  return plane_advection(c, c->p.d.pad, advection, levels, psi, q, w, th, Aq, Aw, Ath, ws, ws_bytes, stream);
+}
+
+int nhqg_sponge_product_ws(nhqg_ctx* c, int levels, const void* f, void* out, void* ws, size_t ws_bytes,
+                           void* stream) {
+  if (!c) return NHQG_ERR_BAD_ARG;
+  return plane_sponge(c, c->p.d.pad, levels, f, out, ws, ws_bytes, stream);
 }
 
 }  // extern "C"

@@ -107,6 +107,7 @@ class Engine:
         nat.check(self.lib.nhqg_ctx_create(ctypes.byref(d), ctypes.byref(handle)), "nhqg_ctx_create")
         self.handle = handle
         self.precision = "fp64"
+        self._plane_bytes: dict[tuple[int, int], int] = {}
         self._finalizer = weakref.finalize(self, Engine._destroy, self.lib, handle.value)
 
     @staticmethod
@@ -226,13 +227,31 @@ class Engine:
         s = self.state_desc(q, w, th, tb)
         nat.check(self.lib.nhqg_sanitize(self.handle, ctypes.byref(s), _stream_handle()), "nhqg_sanitize")
 
+    def _plane_workspace(self, kind: int, levels: int):
+        """(tensor, bytes) lent to a plane product of ``levels`` levels, from
+        torch's allocator on the current stream; none under a capture or where
+        the memory is short (the product then runs in chunks of levels)."""
+        n = self._plane_bytes.get((kind, levels))
+        if n is None:
+            size = ctypes.c_size_t()
+            nat.check(self.lib.nhqg_plane_workspace_bytes(self.handle, kind, levels, ctypes.byref(size)),
+                      "nhqg_plane_workspace_bytes")
+            n = self._plane_bytes[kind, levels] = size.value
+        if n == 0 or torch.cuda.is_current_stream_capturing():
+            return None, 0
+        try:
+            return torch.empty(n, dtype=torch.uint8, device="cuda"), n
+        except torch.cuda.OutOfMemoryError:
+            return None, 0
+
     def triple_advection(self, advection: str, psi, q, w, th, Aq, Aw, Ath) -> None:
         """The grid's products (2/3 or 3/2 rule) of (levels, Nx, Nk) planes."""
         levels = int(q.shape[0])
-        name = "nhqg_triple_advection_32" if self.pad32 else "nhqg_triple_advection_23"
-        nat.check(getattr(self.lib, name)(
+        ws, n = self._plane_workspace(nat.ADV[advection], levels)
+        nat.check(self.lib.nhqg_triple_advection_ws(
             self.handle, nat.ADV[advection], levels, psi.data_ptr(), q.data_ptr(), w.data_ptr(),
-            th.data_ptr(), Aq.data_ptr(), Aw.data_ptr(), Ath.data_ptr(), _stream_handle()), name)
+            th.data_ptr(), Aq.data_ptr(), Aw.data_ptr(), Ath.data_ptr(), ws.data_ptr() if n else None, n,
+            _stream_handle()), "nhqg_triple_advection_ws")
 
     def diagnostics(self, q, w, th, tb) -> torch.Tensor:
         """NHQG_DIAG_COUNT doubles on the device (order of _native.DIAG_KEYS)."""
@@ -272,9 +291,11 @@ class Engine:
         return self.tiles()
 
     def sponge_product(self, f, out) -> None:
-        name = "nhqg_sponge_product_32" if self.pad32 else "nhqg_sponge_product_23"
-        nat.check(getattr(self.lib, name)(self.handle, int(f.shape[0]), f.data_ptr(),
-                                          out.data_ptr(), _stream_handle()), name)
+        levels = int(f.shape[0])
+        ws, n = self._plane_workspace(nat.PLANE_SPONGE, levels)
+        nat.check(self.lib.nhqg_sponge_product_ws(
+            self.handle, levels, f.data_ptr(), out.data_ptr(), ws.data_ptr() if n else None, n,
+            _stream_handle()), "nhqg_sponge_product_ws")
 
 
 def _key(grid: Grid) -> tuple:
