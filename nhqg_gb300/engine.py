@@ -37,6 +37,12 @@ def require_cuda() -> None:
         raise RuntimeError("the NHQG GB300 engine needs a CUDA device (no CPU fallback)")
 
 
+def written_out(t: torch.Tensor) -> torch.Tensor:
+    """t, or a copy without torch's lazy conjugate and negative bits: the engine
+    reads the storage."""
+    return t.resolve_conj().resolve_neg() if t.is_conj() or t.is_neg() else t
+
+
 class Engine:
     """Native context built from a Grid; ``closure``/``exchange`` flags of the
     Grid select the stepper, per-operator calls pass them explicitly."""

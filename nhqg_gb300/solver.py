@@ -27,7 +27,7 @@ import numpy as np
 import torch
 
 from . import _native as nat
-from .engine import engine_for, require_cuda
+from .engine import engine_for, require_cuda, written_out
 from .grid import Grid
 
 
@@ -42,8 +42,7 @@ class State(NamedTuple):
 
 def _dev(x, dtype) -> torch.Tensor:
     if isinstance(x, torch.Tensor):
-        # the engine reads the storage: a lazily conjugated or negated view is written out
-        return x.to(device="cuda", dtype=dtype).contiguous().resolve_conj().resolve_neg()
+        return written_out(x.to(device="cuda", dtype=dtype).contiguous())
     return torch.from_numpy(np.ascontiguousarray(np.asarray(x))).to(device="cuda", dtype=dtype)
 
 

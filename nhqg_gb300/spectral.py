@@ -14,7 +14,7 @@ import numpy as np
 import torch
 
 from .config import NHQGConfig
-from .engine import Engine
+from .engine import Engine, written_out
 from .grid import make_grid
 
 _SPECTRAL: dict[tuple, Engine] = {}
@@ -66,7 +66,7 @@ def _planes(x) -> torch.Tensor:
         t = torch.from_numpy(np.ascontiguousarray(np.asarray(x, dtype=np.complex128))).to("cuda")
     if t.dim() == 2:
         t = t.unsqueeze(0)
-    return t.contiguous().resolve_conj().resolve_neg()
+    return written_out(t.contiguous())
 
 
 def _host(a):
