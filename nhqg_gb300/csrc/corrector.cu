@@ -332,11 +332,17 @@ __device__ __forceinline__ void copy_block(T* __restrict__ dst, const T* __restr
 }
 
 constexpr int kRefine = 2;
-// dynamic shared memory of k_corr_tstep, doubles: vectors, constant tables and
-// the banded inverse (which stays in global memory where it does not fit)
+// dynamic shared memory of k_corr_tstep, doubles: vectors, the transfer tables (rows of
+// ew entries, as many as the caller's matrices have) and the banded inverse; the last
+// two stay in global memory where they do not fit
 __host__ __device__ constexpr int tstep_base(int P, int ew) { return 21 * P + 3 * ew * P + 16; }
 __host__ __device__ constexpr int tstep_inv(int P, int ov) { return ((2 * ov + 1) * P + 1) / 2; }
-constexpr int kTstepMax = 25000;  // 200 KB
+constexpr int kTstepMax = 25000;  // 200 KB; the vectors of 1024 levels take 172 KB
+// entries per row of the tables that are staged
+__host__ __device__ constexpr int tstep_ew(int P, int ew) { return tstep_base(P, ew) <= kTstepMax ? ew : 0; }
+__host__ __device__ constexpr bool tstep_inv_fits(int P, int ew, int ov) {
+  return tstep_base(P, tstep_ew(P, ew)) + tstep_inv(P, ov) <= kTstepMax;
+}
 // at least one thread per level (a 257th row on 256 threads would double every
 // phase), and 256 for the copies
 constexpr int kTstepThreads = 512;
@@ -369,11 +375,17 @@ __global__ void __launch_bounds__(kTstepThreads) k_corr_tstep(CK k, double* vec,
   float* W = reinterpret_cast<float*>(smem + 11 * P + P / 2 + 4);  // fallback: global LU, forward sweep
   double* D1s = smem + 15 * P + 8;                        // [3][P]
   double* Fb = D1s + 3 * P;                               // [2][P] bcF
-  double* tab = smem + tstep_base(P, 0);                  // s2c, c2s values [ew][P] each, then columns
-  int* tabc = reinterpret_cast<int*>(tab + 2 * ew * P);
-  const bool inv_smem = tstep_base(P, ew) + tstep_inv(P, ov) <= kTstepMax;
+  // s2c, c2s values [ew][P] each, then columns
+  const int ews = tstep_ew(P, ew);
+  double* const tab = smem + tstep_base(P, 0);
+  int* const tabc = reinterpret_cast<int*>(tab + 2 * ews * P);
+  const double* const s2c_v = ews ? tab : k.s2c_eval;
+  const double* const c2s_v = ews ? tab + ew * P : k.c2s_eval;
+  const int* const s2c_c = ews ? tabc : k.s2c_ecol;
+  const int* const c2s_c = ews ? tabc + ew * P : k.c2s_ecol;
+  const bool inv_smem = tstep_inv_fits(P, ew, ov);
   float* const Mg = reinterpret_cast<float*>(vec + cv.inv());
-  float* const Ms = inv_smem ? reinterpret_cast<float*>(smem + tstep_base(P, ew)) : Mg;
+  float* const Ms = inv_smem ? reinterpret_cast<float*>(smem + tstep_base(P, ews)) : Mg;
   double* tbs = vec + cv.tb_sbp();
   const double* Bg = vec + cv.Bband();
   // constant tables and what kernels before the previous one left (the previous
@@ -381,10 +393,10 @@ __global__ void __launch_bounds__(kTstepThreads) k_corr_tstep(CK k, double* vec,
   auto stage = [&] {
     copy_block(D1s, k.D1b, 3 * P);
     copy_block(Fb, k.bcF, 2 * P);
-    copy_block(tab, k.s2c_eval, ew * P);
-    copy_block(tab + ew * P, k.c2s_eval, ew * P);
-    copy_block(tabc, k.s2c_ecol, ew * P);
-    copy_block(tabc + ew * P, k.c2s_ecol, ew * P);
+    copy_block(tab, k.s2c_eval, ews * P);
+    copy_block(tab + ews * P, k.c2s_eval, ews * P);
+    copy_block(tabc, k.s2c_ecol, ews * P);
+    copy_block(tabc + ews * P, k.c2s_ecol, ews * P);
     copy_block(xs, tbs, P);
     if (!init) {
       copy_block(A, vec + cv.Aband(), 5 * P);
@@ -579,9 +591,9 @@ __global__ void __launch_bounds__(kTstepThreads) k_corr_tstep(CK k, double* vec,
     u[i] = xs[i] + sol[i];
     double acc = 0.0;
     for (int q = 0; q < ew; ++q) {
-      const int c = tabc[q * P + i];
+      const int c = s2c_c[q * P + i];
       const double v = (c == 0 || c == P - 1) ? 0.0 : sol[c];
-      acc = fma(tab[q * P + i], v, acc);
+      acc = fma(s2c_v[q * P + i], v, acc);
     }
     y[i] = acc;
     t2[i] = acc;
@@ -633,7 +645,7 @@ __global__ void __launch_bounds__(kTstepThreads) k_corr_tstep(CK k, double* vec,
     for (int i = threadIdx.x; i < P; i += blockDim.x) {  // tb_sbp = c2s u
       double acc = 0.0;
       for (int q = 0; q < ew; ++q)
-        acc = fma(tab[(ew + q) * P + i], u[tabc[(ew + q) * P + i]], acc);
+        acc = fma(c2s_v[q * P + i], u[c2s_c[q * P + i]], acc);
       tbs[i] = acc;
     }
   }
@@ -1085,8 +1097,8 @@ cudaError_t run_corrector(const Params& p, const Tables& t, Work& w, const CorrA
     k.win_ov = ov <= CV::kOvMax ? ov : 0;
     if (p.corr_win_ov >= 0) k.win_ov = p.corr_win_ov <= CV::kOvMax ? p.corr_win_ov : 0;
   }
-  int tsd = tstep_base(p.d.P, k.ell_w);
-  if (tsd + tstep_inv(p.d.P, k.win_ov) <= kTstepMax) tsd += tstep_inv(p.d.P, k.win_ov);
+  int tsd = tstep_base(p.d.P, tstep_ew(p.d.P, k.ell_w));
+  if (tstep_inv_fits(p.d.P, k.ell_w, k.win_ov)) tsd += tstep_inv(p.d.P, k.win_ov);
   const size_t tsm = (size_t)tsd * sizeof(double);
   cudaFuncSetAttribute(k_corr_tstep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
   const size_t tsw = (size_t)kTstepSmem(p.d.P) * sizeof(double);
