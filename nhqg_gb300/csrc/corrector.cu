@@ -1104,14 +1104,16 @@ cudaError_t run_corrector(const Params& p, const Tables& t, Work& w, const CorrA
   const size_t tsw = (size_t)kTstepSmem(p.d.P) * sizeof(double);
   if (df) cudaFuncSetAttribute(k_corr_tstep_win, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsw);
   Profiler& pf = w.prof;
+  cudaError_t err = cudaSuccess;  // the first launch that failed; the launchers clear the runtime's
+  auto ck = [&](cudaError_t e) { if (err == cudaSuccess) err = e; };
   pf.begin("corr_pre", st);
-  NHQG_BY_TM(p, CorrColumnOps, pre(p, t, a, df, w.vec + cv.tb_sbp(), st));
+  ck(NHQG_BY_TM(p, CorrColumnOps, pre(p, t, a, df, w.vec + cv.tb_sbp(), st)));
   pf.end(st);
   pf.begin("parseval", st);
   if (df)
-    launch_parseval2(p, wsbp_f, wsbp_f, a.tsbp, p.d.P, w.vec + cv.w2(), w.vec + cv.flux(), w, st, true);
+    ck(launch_parseval2(p, wsbp_f, wsbp_f, a.tsbp, p.d.P, w.vec + cv.w2(), w.vec + cv.flux(), w, st, true));
   else
-    launch_parseval2(p, a.wsbp, a.wsbp, a.tsbp, p.d.P, w.vec + cv.w2(), w.vec + cv.flux(), w, st, false);
+    ck(launch_parseval2(p, a.wsbp, a.wsbp, a.tsbp, p.d.P, w.vec + cv.w2(), w.vec + cv.flux(), w, st, false));
   pf.end(st);
   int n = 2;
   // the double-float path takes the next substep's flux from the fused
@@ -1124,41 +1126,43 @@ cudaError_t run_corrector(const Params& p, const Tables& t, Work& w, const CorrA
     const bool from_mid = s > 0 && mid_flux;
     if (s > 0 && !from_mid) {
       pf.begin("parseval", st);
-      if (df) launch_parseval(p, wsbp_f, a.tsbp, p.d.P, w.vec + cv.flux(), w, st, true);
-      else launch_parseval(p, a.wsbp, a.tsbp, p.d.P, w.vec + cv.flux(), w, st, false);
+      if (df) ck(launch_parseval(p, wsbp_f, a.tsbp, p.d.P, w.vec + cv.flux(), w, st, true));
+      else ck(launch_parseval(p, a.wsbp, a.tsbp, p.d.P, w.vec + cv.flux(), w, st, false));
       pf.end(st);
       ++n;
     }
     pf.begin("corr_step_1d", st);
     if (from_mid)
-      launch_after(k_corr_tstep_win, p.d.P, NT, tsw, st, k, w.vec, sub_dt, last, 0, w.mid_part, nmid, 1.0 / (n2 * n2),
-                   w.counters + p.d.P);
+      ck(launch_after(k_corr_tstep_win, p.d.P, NT, tsw, st, k, w.vec, sub_dt, last, 0, w.mid_part, nmid,
+                      1.0 / (n2 * n2), w.counters + p.d.P));
     else if (df)
-      launch_after(k_corr_tstep_win, 1, NT, tsw, st, k, w.vec, sub_dt, last, s == 0, nullptr, 0, 0.0, nullptr);
+      ck(launch_after(k_corr_tstep_win, 1, NT, tsw, st, k, w.vec, sub_dt, last, s == 0, nullptr, 0, 0.0, nullptr));
     else
-      launch_after(k_corr_tstep, 1, tstep_threads(p.d.P), tsm, st, k, w.vec, sub_dt, last, s == 0);
+      ck(launch_after(k_corr_tstep, 1, tstep_threads(p.d.P), tsm, st, k, w.vec, sub_dt, last, s == 0));
     pf.end(st);
     if (!last && fused_mid && (!df || t.R_val_df)) {
       pf.begin("corr_sub_mid", st);
       if (df) {
         SubK<dfl> sk{p.d.P, p.d.M, t.R_w, t.R_col, t.R_val_df, t.Fs_df, t.Us_df, w.vec + cv.g_half(),
                      dfl(sub_dt)};
-        launch_after(k_corr_sub_mid<cdfl, float2>, nmid, kSubThreads, smid, st, sk, a.tsbp, wsbp_f,
-                                                                      mid_flux ? w.mid_part : nullptr, t.pwt);
+        ck(launch_after(k_corr_sub_mid<cdfl, float2>, nmid, kSubThreads, smid, st, sk, a.tsbp, wsbp_f,
+                        mid_flux ? w.mid_part : nullptr, t.pwt));
       } else {
         SubK<double> sk{p.d.P, p.d.M, t.R_w, t.R_col, t.R_val, t.Fs, t.Us, w.vec + cv.g_half(), sub_dt};
-        launch_after(k_corr_sub_mid<double2, double2>, nmid, kSubThreads, smid, st, sk, a.tsbp, a.wsbp, nullptr, nullptr);
+        ck(launch_after(k_corr_sub_mid<double2, double2>, nmid, kSubThreads, smid, st, sk, a.tsbp, a.wsbp, nullptr,
+                        nullptr));
       }
       pf.end(st);
     } else {
       pf.begin(last ? "corr_sub_last" : "corr_sub", st);
-      NHQG_BY_TM(p, CorrColumnOps, sub(p, t, a, df, w.vec + cv.g_half(), sub_dt, last, w.vec + cv.tmp2(), st));
+      ck(NHQG_BY_TM(p, CorrColumnOps, sub(p, t, a, df, w.vec + cv.g_half(), sub_dt, last, w.vec + cv.tmp2(), st)));
       pf.end(st);
     }
     n += 2;
   }
   if (nlaunch) *nlaunch += n;
-  return cudaGetLastError();
+  ck(cudaGetLastError());
+  return err;
 }
 
 cudaError_t launch_corr_pre(const Params& p, const Tables& t, const double2* w, const double2* th,
