@@ -285,7 +285,6 @@ cudaError_t launch_closure_apply(const Params& p, const Tables& t, const Closure
   if (!cm.w) return cudaErrorInvalidValue;
   ColIn c{p.d.M, p.d.Mc, cm.ncoef, q, t.kx, t.ky, t.inv_denom, cm.sq, cm.se, cm.kmax};
   const size_t sm = sizeof(SmemFwd);
-  cudaFuncSetAttribute(k_closure_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   launch_after(k_closure_apply, (p.d.M + kColsPerCta - 1) / kColsPerCta, kThreads, sm, st, 
       c, reinterpret_cast<const __nv_bfloat16*>(cm.w), cm.s, p.d.P, cq);
   return cudaGetLastError();
@@ -318,7 +317,7 @@ int nhqg_closure_train_step(const void* w_bf16, float* w_master, float* adam_m, 
   Batch b{batch, x, reinterpret_cast<const float2*>(q), reinterpret_cast<const float2*>(target),
           out_scale, 1.f / ((float)batch * target_norm)};
   const size_t sm = sizeof(SmemTrain);
-  cudaFuncSetAttribute(k_closure_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  allow_smem(k_closure_train, sm);
   auto* wb = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(w_bf16));
   k_closure_train<<<(batch + kColsPerCta - 1) / kColsPerCta, kThreads, sm, st>>>(b, wb, grad, loss);
   if (lr > 0.f) {

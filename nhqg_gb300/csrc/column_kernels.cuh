@@ -520,14 +520,12 @@ cudaError_t vfwd_t(const Params& p, const Tables& t, const double2* q, const dou
                    const double2* th, CO* qn, CO* wn, CO* tn, cudaStream_t st) {
   VK k = make_vk(p, t);
   const size_t sm = vsmem<TM>(p, 2, true, sizeof(CO) == sizeof(float2));
-  cudaFuncSetAttribute(k_vfwd<TM, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   launch_after(k_vfwd<TM, CO>, vgrid<TM>(p), NT, sm, st, k, q, w, th, qn, wn, tn);
   return cudaGetLastError();
 }
 
 template <int TM, int MODE, int AK, typename C = double2>
 void vback_t(const VK& k, const VArgs& a, size_t sm, int grid, cudaStream_t st) {
-  cudaFuncSetAttribute(k_vback<TM, MODE, AK, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   launch_after(k_vback<TM, MODE, AK, C>, grid, NT, sm, st, k, a);
 }
 template <int TM, int MODE>
@@ -580,7 +578,6 @@ cudaError_t ColumnOps<TM>::vpost(const Params& p, const Tables& t, const double2
   VK k = make_vk(p, t);
   const size_t sm = vsmem<TM>(p, 3);
   auto kern = df ? k_vpost<TM, cdfl> : k_vpost<TM, double2>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   launch_after(kern, vgrid<TM>(p), NT, sm, st, k, Rq, Rt, w_new, q_out, t_out, zero_mean);
   return cudaGetLastError();
 }
@@ -591,7 +588,6 @@ cudaError_t ColumnOps<TM>::itend(const Params& p, const Tables& t, const double2
   using namespace colk;
   VK k = make_vk(p, t);
   const size_t sm = vsmem<TM>(p, 4);
-  cudaFuncSetAttribute(k_itend<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   launch_after(k_itend<TM>, vgrid<TM>(p), NT, sm, st, k, q, w, th, Iq, Iw, It);
   return cudaGetLastError();
 }

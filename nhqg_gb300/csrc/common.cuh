@@ -24,9 +24,29 @@ namespace nhqg {
 // waiting CTAs take the SMs' slots.
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Lets a kernel take `bytes` of dynamic shared memory.  The limit belongs to the
+// function, not to the launch: setting it to each launch's own size let a thread with
+// a smaller launch of the same kernel lower it between another's call and launch,
+// which then failed.  It is only ever set to one of two values that cover the launch,
+// 200 KB, or all that the kernel's static shared memory leaves.
+template <typename... P>
+inline cudaError_t allow_smem(void (*kern)(P...), size_t bytes) {
+  if (bytes <= 32 * 1024) return cudaSuccess;  // within the default 48 KB, static part included
+  int lim = 200 * 1024;
+  if (bytes > (size_t)lim) {
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+    if (e != cudaSuccess) return e;
+    lim = 227 * 1024 - (int)fa.sharedSizeBytes;
+  }
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+}
+
 template <typename... P, typename... A>
 inline cudaError_t launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                 A&&... args) {
+  const cudaError_t e = allow_smem(kern, smem);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = block;

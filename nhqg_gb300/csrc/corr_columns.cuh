@@ -229,7 +229,6 @@ cudaError_t CorrColumnOps<TM>::pre(const Params& p, const Tables& t, const CorrA
   if (tb_sbp == nullptr) k.c2sV = nullptr;  // no mean-temperature side job
   const size_t sm = 2 * (size_t)p.d.P * TM * sizeof(double2) + col::Cols<TM>::dct_smem_bytes(k.dct);
   auto kern = df ? colk::k_corr_pre<TM, cdfl> : colk::k_corr_pre<TM, double2>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   launch_after(kern, (p.d.M + TM - 1) / TM, col::NT, sm, st, k, a.wp, a.tp, a.wcgl, a.wsbp, a.wcgl_f,
                                                    reinterpret_cast<float2*>(a.wsbp), a.tsbp, a.tbp, tb_sbp);
   return cudaGetLastError();
@@ -244,13 +243,11 @@ cudaError_t CorrColumnOps<TM>::sub(const Params& p, const Tables& t, const CorrA
   const int grid = (p.d.M + TM - 1) / TM;
   if (df) {
     auto kern = colk::k_corr_sub<TM, cdfl, float2>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    launch_after(kern, grid, col::NT, sm, st, k, a.tsbp, reinterpret_cast<const float2*>(a.wsbp), g_half, sub_dt, last,
+      launch_after(kern, grid, col::NT, sm, st, k, a.tsbp, reinterpret_cast<const float2*>(a.wsbp), g_half, sub_dt, last,
                                     a.t_out, a.tcgl_f, y_mean, a.tb_out);
   } else {
     auto kern = colk::k_corr_sub<TM, double2, double2>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    launch_after(kern, grid, col::NT, sm, st, k, a.tsbp, a.wsbp, g_half, sub_dt, last, a.t_out, a.tcgl, y_mean, a.tb_out);
+      launch_after(kern, grid, col::NT, sm, st, k, a.tsbp, a.wsbp, g_half, sub_dt, last, a.t_out, a.tcgl, y_mean, a.tb_out);
   }
   return cudaGetLastError();
 }

@@ -1082,11 +1082,6 @@ cudaError_t run_corrector(const Params& p, const Tables& t, Work& w, const CorrA
   float2* wsbp_f = reinterpret_cast<float2*>(a.wsbp);
   const size_t smid = (size_t)p.d.P * kSM * sizeof(double2);
   const bool fused_mid = smid <= 200 * 1024 && t.R_col != nullptr;
-  if (fused_mid) {
-    cudaFuncSetAttribute(k_corr_sub_mid<double2, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smid);
-    cudaFuncSetAttribute(k_corr_sub_mid<cdfl, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smid);
-  }
   {  // reach of the banded inverse: r^ov <= 1e-7 for the decay rate r of A^-1 (two rows of margin)
     const double aa = 0.5 * k.mu * k.kappa * sub_dt * (double)p.d.Nz * (double)p.d.Nz;
     int ov = 2;
@@ -1100,9 +1095,7 @@ cudaError_t run_corrector(const Params& p, const Tables& t, Work& w, const CorrA
   int tsd = tstep_base(p.d.P, tstep_ew(p.d.P, k.ell_w));
   if (tstep_inv_fits(p.d.P, k.ell_w, k.win_ov)) tsd += tstep_inv(p.d.P, k.win_ov);
   const size_t tsm = (size_t)tsd * sizeof(double);
-  cudaFuncSetAttribute(k_corr_tstep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsm);
   const size_t tsw = (size_t)kTstepSmem(p.d.P) * sizeof(double);
-  if (df) cudaFuncSetAttribute(k_corr_tstep_win, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsw);
   Profiler& pf = w.prof;
   cudaError_t err = cudaSuccess;  // the first launch that failed; the launchers clear the runtime's
   auto ck = [&](cudaError_t e) { if (err == cudaSuccess) err = e; };

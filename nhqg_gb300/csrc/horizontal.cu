@@ -484,9 +484,6 @@ cudaError_t launch_horizontal_t(const Params& p, const HTables<C>& t, Work& w, c
   size_t sm3 = tb + (size_t)k.ng * CB3 * seqb;
   if (sm3 > budget) return cudaErrorInvalidConfiguration;
 
-  cudaFuncSetAttribute(k_h1<C, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-  cudaFuncSetAttribute(k_h2<C, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-  cudaFuncSetAttribute(k_h3<C, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
   dim3 g1((k.cols_in + CB1 - 1) / CB1, a.levels);
   w.prof.begin(sizeof(T) == 4 ? "h1_col_ifft_f32" : "h1_col_ifft", st);
   launch_after(k_h1<C, CI>, g1, 256, sm1, st, k, CB1);
@@ -558,8 +555,6 @@ cudaError_t launch_phys_maxima(const Params& p0, const Tables& t, Work& w, const
   while (RB * 2 <= 16 && k.N % (RB * 2) == 0 && tb + (size_t)4 * (RB * 2 / 2) * seqb <= 96 * 1024) RB *= 2;
   const size_t sm2 = tb + (size_t)4 * (RB / 2) * seqb;
   if (sm1 > budget || sm2 > budget) return cudaErrorInvalidConfiguration;
-  cudaFuncSetAttribute(k_h1<double2, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
-  cudaFuncSetAttribute(k_hmax, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
   w.prof.begin("diag_maxima", st);
   launch_after(k_h1<double2, double2>, dim3((k.cols_in + CB1 - 1) / CB1, k.levels), 256, sm1, st, k, CB1);
   launch_after(k_hmax, dim3(k.N / RB, k.levels), 256, sm2, st, k, RB, maxima);

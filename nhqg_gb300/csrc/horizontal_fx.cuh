@@ -779,10 +779,6 @@ cudaError_t launch(const HX& args, cudaStream_t st, Profiler& prof) {
   const size_t sm3 = head + (size_t)k.Mr * (CB + 1) * sizeof(double2);
   auto h2 = k_h2x<F, HF_JAC, false>;
   if (k.form == HF_FLUX) h2 = k.sponge ? k_h2x<F, HF_FLUX, true> : k_h2x<F, HF_FLUX, false>;
-  cudaError_t e = cudaFuncSetAttribute(k_h1x<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(h2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_h3x<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
-  if (e != cudaSuccess) return e;
   prof.begin("h1_col_ifft", st);
   launch_after(k_h1x<F>, dim3(c1, k.levels, 4 / k.stage), 32 * F::W, sm1, st, k);
   prof.end(st);

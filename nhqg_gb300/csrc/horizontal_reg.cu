@@ -718,14 +718,11 @@ cudaError_t launch_reg(const HR& k, cudaStream_t st, Profiler& prof) {
   const size_t cap = 200 * 1024;
   if (sm1 > cap || sm2 > cap || sm3 > cap) return cudaErrorInvalidConfiguration;
   auto h1 = z1 > 1 ? k_h1r<R1, R2, true> : k_h1r<R1, R2, false>;
-  cudaFuncSetAttribute(h1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
   // the SP instantiations carry the sponge and the gradient-form eta terms
   const bool sp = k.sponge || k.eta_grad;
   auto h2 = k_h2r<R1, R2, HF_SPONGE, true>;
   if (k.form == HF_FLUX) h2 = sp ? k_h2r<R1, R2, HF_FLUX, true> : k_h2r<R1, R2, HF_FLUX, false>;
   else if (k.form == HF_JAC) h2 = sp ? k_h2r<R1, R2, HF_JAC, true> : k_h2r<R1, R2, HF_JAC, false>;
-  cudaFuncSetAttribute(h2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
-  cudaFuncSetAttribute(k_h3r<R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
   prof.begin("h1_col_ifft_f32", st);
   launch_after(h1, dim3(c1, k.levels, z1), 128, sm1, st, k);
   prof.end(st);

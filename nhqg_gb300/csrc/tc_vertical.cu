@@ -502,12 +502,8 @@ namespace {
 template <bool INV>
 cudaError_t tc_launch(const TcArgs& a, int nf, cudaStream_t st) {
   const size_t sm = tc_smem<INV>();
-  cudaError_t e = cudaFuncSetAttribute(k_tc_vertical<INV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sm);
-  if (e != cudaSuccess) return e;
   dim3 grid((a.ncols + kCols - 1) / kCols, nf);
-  launch_after(k_tc_vertical<INV>, grid, kThreads + 64, sm, st, a);
-  return cudaGetLastError();
+  return launch_after(k_tc_vertical<INV>, grid, kThreads + 64, sm, st, a);
 }
 }  // namespace
 

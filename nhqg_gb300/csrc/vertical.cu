@@ -445,7 +445,6 @@ cudaError_t launch_shell(const Params& p, const Tables& t, const Work& w, const 
                          double2* w_out, cudaStream_t st) {
   if (t.shell_fx) return launch_shell_tc(p, t, w, rhs_w, w_out, st);
   const size_t sm = (size_t)p.d.G * SHELL_NC * sizeof(double2);
-  cudaFuncSetAttribute(k_shell, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   launch_after(k_shell, t.n_shells, NT, sm, st, t.shell_inv, t.shell_start, t.shell_modes, rhs_w, w_out,
                                       p.d.G, p.d.M);
   return cudaGetLastError();
