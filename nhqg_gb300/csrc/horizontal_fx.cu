@@ -15,7 +15,7 @@ cudaError_t launch_hfx_144(const hfx::HX&, cudaStream_t, Profiler&);
 cudaError_t launch_hfx_192(const hfx::HX&, cudaStream_t, Profiler&);
 cudaError_t launch_hfx_256(const hfx::HX&, cudaStream_t, Profiler&);
 
-// Lengths R L in three register stages (hfx::Lane), at most 32 lanes of 16 values;
+// Lengths R L in three register stages (hfx::Lane), at most 32 lanes of 8 or 12 values;
 // others (longer ones, and the tiny test grids) keep the FP64 kernels of
 // horizontal.cu.
 bool horizontal_fx_supported(int N) {

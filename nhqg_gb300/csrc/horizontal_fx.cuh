@@ -291,8 +291,7 @@ __device__ __forceinline__ int align(cfx* z, const int* e) {
   unsigned s = 0;
   sfor<NE>([&](auto ii) {
     constexpr int i = decltype(ii)::value;
-    const long long ax = z[i].x < 0 ? -z[i].x : z[i].x, ay = z[i].y < 0 ? -z[i].y : z[i].y;
-    s += ((((unsigned)(ax >> 32) >> 8) + ((unsigned)(ay >> 32) >> 8)) >> min(31, em - e[i])) + 1u;
+    s += cterm(z[i], min(31, em - e[i]));
   });
   s = gsum<LS>(s);
   const int E = max(em, em - (kBits - 40) + bitlen(s));
