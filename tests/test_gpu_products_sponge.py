@@ -1,4 +1,5 @@
-"""Sponge and trap terms of the fixed-point products: non-finite sponge values."""
+"""Sponge and trap terms of the fixed-point products at every transform length: the
+explicit tendency against the oracle, and non-finite sponge values."""
 
 import numpy as np
 import pytest
@@ -35,6 +36,22 @@ def _grid(nx, rule, eta=0.0, seed=0):
 def _state(g, mask, seed=1):
     rng = np.random.default_rng(seed)
     return (*(np.fft.rfft2(rng.standard_normal((lv, g.Nx, g.Nx))) * mask for lv in (5, 3, 3)), np.zeros(5))
+
+
+# transform lengths 48, 64, 96, 128, 192 and the padded 72, 96, 144, 192; a background PV
+# 1e4 times q has to cancel out of the sponge's operand
+@pytest.mark.parametrize("nx,rule", [(48, "23"), (64, "23"), (96, "23"), (128, "23"), (192, "23"),
+                                     (48, "32"), (64, "32"), (96, "32"), (128, "32")])
+@pytest.mark.parametrize("eta", [0.0, 1.0, 1e4])
+def test_against_oracle(nx, rule, eta):
+    import oracle
+    from nhqg_gb300 import solver as S
+    g, o = _grid(nx, rule, eta)
+    s = _state(g, o.mask_23)
+    ref = oracle.nhqg_oracle.explicit_rhs(oracle.nhqg_oracle.OracleState(*s), o)
+    for got, want in zip(S.explicit_rhs(s, g)[:3], ref[:3]):
+        # the operators' bound; with the trap the tendency of q is of its advection's size
+        assert np.linalg.norm(got.cpu().numpy() - want) <= 1e-12 * np.linalg.norm(want)
 
 
 @pytest.mark.parametrize("nx,rule", [(48, "23"), (64, "23"), (48, "32")])
