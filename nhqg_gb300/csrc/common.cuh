@@ -17,8 +17,11 @@ namespace nhqg {
 // the next grid to the GPU before the previous one has ended, and its CTAs,
 // which start as the previous grid's leave, wait in after_previous() (all of that
 // grid done, its writes visible) before they touch anything a kernel writes.
-// Every kernel launched that way calls it, so completion stays ordered along the
-// stream; only constant tables are read before it.  Per step: 64^2 x 32 plain 661
+// Every CTA of every kernel launched that way calls it, so completion stays ordered
+// along the stream.  Before it a kernel may read constant tables, and what a kernel
+// before the previous one left: its CTAs start when every CTA of the previous grid has
+// exited, each of which had waited for the grid before that.  k_corr_tstep alone does the
+// latter (run_corrector states the order it needs).  Per step: 64^2 x 32 plain 661
 // -> 570 us, 96^2 x 48 mixed 600 -> 520.  Letting the next grid in early
 // (launch_dependents at the start of each kernel) measured 726 and 665: its
 // waiting CTAs take the SMs' slots.

@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kTstepThreads) k_corr_tstep(CK k, double* vec,
   double* tbs = vec + cv.tb_sbp();
   const double* Bg = vec + cv.Bband();
   // constant tables and what kernels before the previous one left (the previous
-  // kernel writes the flux and <w^2> only): A, the banded inverse, tb_sbp
+  // kernel, a Parseval sum, writes the flux and <w^2> only): A, the banded inverse, tb_sbp
   auto stage = [&] {
     copy_block(D1s, k.D1b, 3 * P);
     copy_block(Fb, k.bcF, 2 * P);
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kTstepThreads) k_corr_tstep(CK k, double* vec,
     for (int e = 0; e < 3; ++e) {
       const int c = min(max(i - 1 + e, 0), P - 1);
       dv[e] = d1at(e, i);
-      fv[e] = __ldcg(flux + c);  // written by other CTAs of this launch
+      fv[e] = __ldcg(flux + c);
     }
     double acc = 0.0;
 #pragma unroll
@@ -1124,6 +1124,9 @@ cudaError_t run_corrector(const Params& p, const Tables& t, Work& w, const CorrA
       pf.end(st);
       ++n;
     }
+    // k_corr_tstep reads tb_sbp, A and the banded inverse ahead of its wait: the kernel
+    // launched just before it has to be one that writes none of them (the Parseval sum
+    // above; tb_sbp comes from k_corr_pre or the last k_corr_tstep)
     pf.begin("corr_step_1d", st);
     if (from_mid)
       ck(launch_after(k_corr_tstep_win, p.d.P, NT, tsw, st, k, w.vec, sub_dt, last, 0, w.mid_part, nmid,
