@@ -469,10 +469,14 @@ __global__ void __launch_bounds__(32 * F::W, F::L == 32 ? 2 : 1) k_h1x(HX k) {
     });
     em = gmax<LS>(em);
     // columns of zeros (planes beyond the 2/3 band) need no transform: their
-    // exponent tells H2 so
+    // exponent tells H2 so (1 is the exponent of the subnormals too)
     if (__all_sync(kFull, em == 1)) {
-      if (live && l == 0) k.e1[((size_t)f * k.levels + lev) * k.cols_in + c] = kEZero;
-      continue;
+      unsigned long long any = 0;
+      sfor<R>([&](auto jj) { any |= dbits(v[decltype(jj)::value].x) | dbits(v[decltype(jj)::value].y); });
+      if (!__any_sync(kFull, (any << 1) != 0)) {
+        if (live && l == 0) k.e1[((size_t)f * k.levels + lev) * k.cols_in + c] = kEZero;
+        continue;
+      }
     }
     unsigned s = 0;
     sfor<R>([&](auto jj) {
