@@ -30,7 +30,7 @@
 //
 // Measured, one evaluation: 256^2 x 257 levels 8.8 -> 2.1 ms (H1 1.51 -> 0.43,
 // H2 5.53 -> 1.07, H3 1.73 -> 0.60), 192^2 x 97 2.09 -> 0.66, 128^2 x 81 under the
-// 3/2 rule 1.73 -> 0.65, full planes 256^2 x 65 2.56 -> 0.65.  H2 issues in 62% of
+// 3/2 rule 1.73 -> 0.65, full planes 256^2 x 65 2.56 -> 0.65.  H2 issues in 60% of
 // the cycles (16 warps per SM, limited by registers and shared memory).
 //
 // Scaling: irfft2's 1/(N Nx) of both factors of a product rides on the
